@@ -730,6 +730,7 @@ int grid_error(minim_gpu_instance_s* h) {
 }
 
 int rule_threads(int kk, const InstDesc& d);
+int lj_batch_rows(const MinParams& mp);
 bool single_shape(int kk, const InstDesc& d, int* threads, int* csize);
 void launch_single(int kk, int threads, int csize, const InstDesc* d_inst, int* counter, const InstDesc& d,
                    cudaStream_t s);
@@ -959,6 +960,8 @@ void do_minimise(minim_gpu_instance_s* h, const minim_gpu_minimiser_params& mp, 
   ws_apply(d, (char*)h->ws, L);
   d.mp = to_mp(mp, tol);
   ws_sched(d, (char*)h->ws, L, sched_of(mp), D.s);
+  // (line searches resolve differences of energies: rows sum them term by term, tiles in plain runs of 32)
+  if (small && h->kk == K_LJ && !lj_batch_rows(d.mp)) d.lj.rows = 2;
   d.stage_bytes = small ? 0 : grid_stage_bytes(h->kk);
   d.pf_dist = small ? 0 : prefetch_cfg();
   d.pf.pf_dist = d.pf_dist;

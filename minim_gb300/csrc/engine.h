@@ -28,7 +28,8 @@ struct PotLJ {
   double inv_cs;   // 1 / cell size (the cell size is rc * (1 + 1e-3))
   int hbits;       // log2 of the hash table's buckets
   int* cells;      // scratch: lj_cell_ints(np, hbits) ints
-  int rows;        // one-CTA evaluators: 1 rows / dealt tile pairs, 0 tile pairs by rounds
+  int rows;        // one-CTA evaluators: 1 rows / dealt tile pairs, 2 the same with FP32 by rows only, 0 tile
+                   // pairs by rounds
   int split;       // energy items per particle, set by the kernel (lj_split)
 };
 #ifdef __CUDACC__
@@ -67,6 +68,7 @@ constexpr int kLjRowsMax = 64;
 constexpr int kLjDealt2Min = 256;
 MG_HD inline bool lj_dealt_fits(int np, int nwarps, bool fp64, int rows) {
   if (!rows) return !fp64 && lj_dealt_bytes(np, nwarps, fp64) <= kLjSmemBudget;
+  if (rows == 2 && !fp64) return false;
   return np > kLjRowsMax && lj_dealt_bytes(np, nwarps, fp64) <= kLjSmemRows;
 }
 // shared memory of a launch for a cluster of np particles with the given

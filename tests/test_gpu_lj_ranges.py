@@ -1,5 +1,5 @@
 """Lennard-Jones evaluators at the ends of their ranges: coordinates in large
-units, sums of many comparable terms.
+units, sums of many comparable terms, energies of very unequal pairs.
 """
 import numpy as np
 import pytest
@@ -88,3 +88,31 @@ def test_energy_sums(n):
         e, _ = inst.energy_gradient(pts.ravel())
         sq += float(((e - eo) / eo) ** 2)
     assert np.sqrt(sq / 200) <= 1.1 * {13: 2.5e-15, 55: 1.4e-15, 64: 1.3e-15, 96: 1.1e-15}[n]
+
+
+def test_fp32_energy_keeps_small_terms():
+    """150 sites 1000 apart, each a pair of particles a quarter apart (energy 4 x
+    16773120, exact in FP32 as is each of its steps) among twelve neighbours of
+    some -0.1 each.  Every pair's own error is at most 1e-6 of |r^-12| + |r^-6|, in
+    all below 15 of each a site; a sum that rounds at 1 loses tenths a site."""
+    ring = np.array([[a, b, 0] for a in (-1, 1) for b in (-1, 1)] + [[a, 0, b] for a in (-1, 1) for b in (-1, 1)]
+                    + [[0, a, b] for a in (-1, 1) for b in (-1, 1)], float)
+    site = np.concatenate([[[0, 0, 0], [0.25, 0, 0]], ring])
+    pts = np.concatenate([site + [1000.0 * k, 0, 0] for k in range(150)])
+    pts = pts[np.argsort(Rng(8).uniform(len(pts)), kind="stable")]
+    d = site[:, None] - site[None]
+    r2 = (d * d).sum(2)[np.triu_indices(len(site), 1)]
+    assert np.sum(r2 ** -6 + r2 ** -3) - (16.0 ** 6 + 16.0 ** 3) < 15
+    exact = 150 * 4 * np.sum(r2 ** -6 - r2 ** -3)
+    inst = runtime.Instance(abi.lj(), pts.ravel())
+    # (sites see one another at 1000 apart: 4e-18 a pair)
+    for gradient in (True, False):
+        e, _ = inst.eval_kernel(abi.EVAL_FP32_GRID, pts.ravel(), gradient=gradient)
+        assert abs(e - exact) <= 150 * 4 * 15 * 1e-6, e - exact
+    # single minimisations' own evaluations, on one CTA and on a cluster (coordinates fixed: the first energy is the last)
+    for sites in (3, 6, 20):
+        some = np.concatenate([site + [1000.0 * k, 0, 0] for k in range(sites)])
+        some = some[np.argsort(Rng(sites).uniform(len(some)), kind="stable")]
+        inst = runtime.Instance(abi.lj(), some.ravel(), fixed=list(range(some.size)))
+        r = inst.minimise(abi.minimiser("lbfgs", tol=1e-9, max_iter=5, precision="fp32"))
+        assert abs(r.energy - exact * sites / 150) <= sites * 4 * 15 * 1e-6, (sites, r.energy)
