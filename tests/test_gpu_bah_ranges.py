@@ -1,10 +1,15 @@
 """BarAndHinge at the ends of its ranges: FP32 forces of very unequal elements
-at one vertex, hinge angles on both sides of their rule.
+at one vertex, hinge angles on both sides of their rule, a vertex of thousands
+of elements.
 """
+import time
+
 import numpy as np
 import pytest
+import torch
 
 from minim_gb300 import abi, runtime
+from tests.workloads import Rng
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +52,45 @@ def test_hinge_angle_on_both_sides_of_its_rule(d0, path):
         want = [0.5 * (d0 - phi) ** 2, 0.5 * (d0 + phi) ** 2]
         tol = 1e-12 * max(phi, abs(d0)) ** 2
         assert np.max(np.abs(np.sort(es) - np.sort(want))) <= tol, (phi, es, want)
+
+
+def _fan(n):
+    a = np.arange(n) * 2 * np.pi / n
+    pts = np.concatenate([[[0, 0, 0.2]], np.stack([np.cos(a) * 3, np.sin(a) * 3, 0.1 * np.cos(5 * a)], 1)])
+    return pts.ravel(), np.array([[0, 1 + i, 1 + (i + 1) % n] for i in range(n)], np.int32)
+
+
+def _exact(bars, bpar, hinges, hpar, x):
+    """Energy and forces in 64 bits, the hinge's angle from pi by an arctangent
+    (the reference's arccosine is good to 1e-8 only where triangles are nearly
+    coplanar, as in a wide fan); its bar force carries a factor of two."""
+    X = torch.from_numpy(x.reshape(-1, 3).copy()).requires_grad_(True)
+    b, h = torch.from_numpy(bars.astype(np.int64)), torch.from_numpy(hinges.astype(np.int64))
+    bp, hp = torch.from_numpy(bpar), torch.from_numpy(hpar)
+    dl = (X[b[:, 0]] - X[b[:, 1]]).norm(dim=1) - bp[:, 1]
+    q = [X[h[:, k]] for k in range(4)]
+    b1, b2, b3 = q[1] - q[0], q[2] - q[1], q[3] - q[2]
+    n1, n2 = torch.linalg.cross(b1, b2), torch.linalg.cross(b2, b3)
+    th = torch.atan2(-b2.norm(dim=1) * (n1 * b3).sum(1), -(n1 * n2).sum(1)) - (hp[:, 1] - np.pi)
+    es, eb = 0.5 * (bp[:, 0] * dl * dl).sum(), 0.5 * (hp[:, 0] * th * th).sum()
+    g, = torch.autograd.grad(2 * es + eb, X)
+    return (es + eb).item(), g.numpy().ravel()
+
+
+@pytest.mark.parametrize("n", [40, 90, 300, 3000])
+def test_hub(n):
+    """A vertex in n triangles has 2 n elements: its list is put in order without
+    a quadratic pass (one thread would take a second at 3000), and the forces
+    are 64-bit arithmetic's to 1e-12, times the triangles' aspect where they are thin."""
+    x, tris = _fan(n)
+    y = x + 0.05 * min(1.0, 40 / n) * (Rng(1).uniform(x.size) - 0.5)
+    b, bp, h, hp = runtime.bah_elements(abi.bar_and_hinge(triangulation=tris, rigidity=(1, 0.1)), x)
+    p = abi.bar_and_hinge(bonds=b, hinges=h, rigidity=(1, 0.1))
+    runtime.Instance(p, x)
+    t = time.perf_counter()
+    inst = runtime.Instance(p, x)
+    assert time.perf_counter() - t < 0.2
+    eo, go = _exact(b, bp, h, hp, y)
+    e, g = inst.energy_gradient(y)
+    tol = 1e-12 * max(1.0, n / 40)
+    assert abs(e - eo) <= tol * abs(eo) and np.max(np.abs(g - go)) <= tol * np.max(np.abs(go))
