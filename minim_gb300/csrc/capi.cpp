@@ -460,6 +460,12 @@ struct minim_gpu_instance_s {
     if (p) owned.push_back(p);
     return p;
   }
+  // the same for one of the potential's arrays of `bytes`, which count against
+  // a server's budget
+  void* own_pot(void* p, size_t bytes) {
+    if (p) pot_bytes += bytes;
+    return own(p);
+  }
   template <typename T>
   T* own_upload(const std::vector<T>& v) {
     T* p = upload(v);
@@ -478,6 +484,14 @@ struct minim_gpu_instance_s {
 
 namespace {
 
+// device-built element lists
+void bah_own(minim_gpu_instance_s* h, const BahTopoDev& T) {
+  h->own_pot(T.bars, T.nbar * sizeof(int2));
+  h->own_pot(T.bpar, T.nbar * sizeof(double2));
+  h->own_pot(T.hinges, T.nhinge * sizeof(int4));
+  h->own_pot(T.hpar, T.nhinge * sizeof(double2));
+}
+
 // The evaluations' form of the current element list, and its element vectors
 void bah_slots(minim_gpu_instance_s* h) {
   PotBAH& P = h->d.bah;
@@ -493,19 +507,20 @@ void bah_slots(minim_gpu_instance_s* h) {
   if (mg_bah_slots_device(bars, bpar, P.nbar, hinges, hpar, P.nhinge, P.nvert, direct ? 0 : 1, &o, dev().s) !=
       MG_TOPO_OK)
     throw ApiError{MINIM_GPU_ERR_CUDA, "BarAndHinge device set-up failed"};
-  P.vbars = o.bars ? (int2*)h->own(o.bars) : bars;
-  P.vbar_pf = (float4*)h->own(o.bar_pf);
-  P.vbar_pd = o.bar_pd ? (double2*)h->own(o.bar_pd) : bpar;
-  P.bar_slot = (int2*)h->own(o.bar_slot);
-  P.vhinges = o.hinges ? (int4*)h->own(o.hinges) : hinges;
-  P.vhinge_pf = (float4*)h->own(o.hinge_pf);
-  P.vhinge_pd = o.hinge_pd ? (double2*)h->own(o.hinge_pd) : hpar;
-  P.vhinge_d0 = (float2*)h->own(o.hinge_d0);
-  P.hinge_slot = (int4*)h->own(o.hinge_slot);
-  P.vert_off = (int*)h->own(o.vert_off);
-  P.vert_deg = (int*)h->own(o.vert_deg);
+  const size_t nb = (size_t)P.nbar, nh = (size_t)P.nhinge, nv = (size_t)P.nvert;
+  P.vbars = o.bars ? (int2*)h->own_pot(o.bars, nb * sizeof(int2)) : bars;
+  P.vbar_pf = (float4*)h->own_pot(o.bar_pf, nb * sizeof(float4));
+  P.vbar_pd = o.bar_pd ? (double2*)h->own_pot(o.bar_pd, nb * sizeof(double2)) : bpar;
+  P.bar_slot = (int2*)h->own_pot(o.bar_slot, nb * sizeof(int2));
+  P.vhinges = o.hinges ? (int4*)h->own_pot(o.hinges, nh * sizeof(int4)) : hinges;
+  P.vhinge_pf = (float4*)h->own_pot(o.hinge_pf, nh * sizeof(float4));
+  P.vhinge_pd = o.hinge_pd ? (double2*)h->own_pot(o.hinge_pd, nh * sizeof(double2)) : hpar;
+  P.vhinge_d0 = (float2*)h->own_pot(o.hinge_d0, nh * sizeof(float2));
+  P.hinge_slot = (int4*)h->own_pot(o.hinge_slot, nh * sizeof(int4));
+  P.vert_off = (int*)h->own_pot(o.vert_off, (nv / 32 + 2) * sizeof(int));
+  P.vert_deg = (int*)h->own_pot(o.vert_deg, nv * sizeof(int));
   P.nslot = o.nslot;
-  P.elem_vec = h->own(dalloc(24 * (size_t)o.nslot));
+  P.elem_vec = h->own_pot(dalloc(24 * (size_t)o.nslot), 24 * (size_t)o.nslot);
 }
 
 // the host's element lists by colour
@@ -573,9 +588,7 @@ void upload_bah_arrays(minim_gpu_instance_s* h) {
     if (!h->fixed.empty()) {
       if (mg_bah_keep_device(&h->bah_topo, h->fixed.data(), &h->bah_kept, dev().s) != MG_TOPO_OK)
         throw ApiError{MINIM_GPU_ERR_CUDA, "BarAndHinge device set-up failed"};
-      for (void* p : {(void*)h->bah_kept.bars, (void*)h->bah_kept.bpar, (void*)h->bah_kept.hinges,
-                      (void*)h->bah_kept.hpar})
-        h->own(p);
+      bah_own(h, h->bah_kept);
       for (int v = 0; v < P.nvert; v++)
         node_el[v] = !(h->fixed[3 * v] && h->fixed[3 * v + 1] && h->fixed[3 * v + 2]);
     }
@@ -668,10 +681,7 @@ minim_gpu_instance_s* create_instance(int kind, const void* params, const double
         if (rc == MG_TOPO_INVALID) throw ApiError{MINIM_GPU_ERR_INVALID, msg};
         if (rc == MG_TOPO_CUDA) throw ApiError{MINIM_GPU_ERR_CUDA, "BarAndHinge device set-up failed"};
         if (rc == MG_TOPO_OK) {
-          h->own(h->bah_topo.bars);
-          h->own(h->bah_topo.bpar);
-          h->own(h->bah_topo.hinges);
-          h->own(h->bah_topo.hpar);
+          bah_own(h, h->bah_topo);
           h->bah = BahHost{};
           h->bah.nvert = (int)(ndof / 3);
           bah_scalars(*q, h->bah);

@@ -1,6 +1,6 @@
 """BarAndHinge at the ends of its ranges: FP32 forces of very unequal elements
 at one vertex, hinge angles on both sides of their rule, a vertex of thousands
-of elements.
+of elements, the memory a request holds.
 """
 import time
 
@@ -9,7 +9,7 @@ import pytest
 import torch
 
 from minim_gb300 import abi, runtime
-from tests.workloads import Rng
+from tests.workloads import Rng, sheet
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +94,25 @@ def test_hub(n):
     e, g = inst.energy_gradient(y)
     tol = 1e-12 * max(1.0, n / 40)
     assert abs(e - eo) <= tol * abs(eo) and np.max(np.abs(g - go)) <= tol * np.max(np.abs(go))
+
+
+@pytest.mark.parametrize("explicit", [False, True])
+def test_server_budget_counts_the_elements(explicit):
+    """The server's memory budget is for what a request keeps on the device: a
+    sheet's element lists and force slots (over 600 bytes a vertex) are more
+    than its minimiser's vectors."""
+    flat, tris, pert = sheet(64, seed=5)
+    p = abi.bar_and_hinge(triangulation=tris, rigidity=(1, 0.01))
+    if explicit:
+        b, _, h, _ = runtime.bah_elements(p, flat)
+        p = abi.bar_and_hinge(bonds=b, hinges=h, rigidity=(1, 0.01))
+    mp = abi.minimiser("lbfgs", m=5, tol=1e-6, max_iter=3)
+    vectors = 3 * 64 * 64 * 4 * (2 * 1 + 2 * 2 + 2 + 2 * 6)
+    for spare, status in ((500, abi.RES_REJECTED), (4000, abi.RES_MAXITER)):
+        srv = runtime.Server(max_bytes=vectors + 20000 + spare * 64 * 64)
+        srv.submit(p, pert if explicit else flat, mp)
+        while srv.step() != (0, 0):
+            pass
+        (_, r), = srv.poll()
+        assert (r.status == abi.RES_REJECTED) == (status == abi.RES_REJECTED)
+        srv.close()
