@@ -429,6 +429,10 @@ struct minim_gpu_instance_s {
   bool bah_coloured = false, bah_col_host = false;
   std::vector<unsigned char> fixed;
   size_t pot_bytes = 0;
+  // what the current element lists hold (bah_collect): freed when other fixed
+  // degrees of freedom make new ones
+  std::vector<void*> bah_owned;
+  size_t bah_bytes = 0;
   // grid-launch resources (lazy)
   InstDesc* d_desc = nullptr;
   EvalIO* d_io = nullptr;
@@ -475,6 +479,7 @@ struct minim_gpu_instance_s {
   }
   ~minim_gpu_instance_s() {
     for (void* p : owned) dfree(p);
+    for (void* p : bah_owned) dfree(p);
     dfree(ws);
     pinned().free(hx, n * sizeof(double));
     pinned().free(h_out, sizeof(EvalOut));
@@ -483,6 +488,14 @@ struct minim_gpu_instance_s {
 };
 
 namespace {
+
+// what the instance has come to own past the first `mark` arrays, with
+// pot_bytes `bytes` before them, belongs to its element lists
+void bah_collect(minim_gpu_instance_s* h, size_t mark, size_t bytes) {
+  h->bah_owned.insert(h->bah_owned.end(), h->owned.begin() + mark, h->owned.end());
+  h->owned.resize(mark);
+  h->bah_bytes += h->pot_bytes - bytes;
+}
 
 // device-built element lists
 void bah_own(minim_gpu_instance_s* h, const BahTopoDev& T) {
@@ -546,6 +559,7 @@ void bah_host_colours(minim_gpu_instance_s* h, const BahDevArrays& A) {
 // set-up.
 void bah_colours(minim_gpu_instance_s* h) {
   if (h->bah_coloured) return;
+  const size_t mark = h->owned.size(), bytes = h->pot_bytes;
   const BahTopoDev& T = h->bah_kept;
   BahColouredDev& C = h->bah_col;
   const int rc = mg_bah_colour_device(&T, &C, dev().s);
@@ -554,6 +568,7 @@ void bah_colours(minim_gpu_instance_s* h) {
     for (void* p : {(void*)C.bars, (void*)C.bpar, (void*)C.bar_off, (void*)C.hinges, (void*)C.hpar,
                     (void*)C.hinge_off})
       h->own(p);
+    bah_collect(h, mark, bytes);
     h->bah_coloured = true;
     return;
   }
@@ -572,12 +587,14 @@ void bah_colours(minim_gpu_instance_s* h) {
   CK(cudaStreamSynchronize(dev().s));
   const BahDevArrays A = bah_arrays(B, {});
   bah_host_colours(h, A);
+  bah_collect(h, mark, bytes);
   CK(cudaStreamSynchronize(dev().s));
 }
 
 void upload_bah_arrays(minim_gpu_instance_s* h) {
   PotBAH& P = h->d.bah;
   P.nvert = h->bah.nvert;
+  const size_t mark = h->owned.size(), bytes = h->pot_bytes;
   // alive until bah_slots has waited for the stream
   BahDevArrays A;
   std::vector<unsigned char> node_el;
@@ -609,6 +626,13 @@ void upload_bah_arrays(minim_gpu_instance_s* h) {
   P.wall_eps = h->bah.wall_eps;
   P.wall_sig = h->bah.wall_sig;
   bah_slots(h);
+  // no work that reads the former lists is in flight: every call waits for its own
+  for (void* p : h->bah_owned) dfree(p);
+  h->bah_owned.clear();
+  const size_t former = h->bah_bytes;
+  h->bah_bytes = 0;
+  bah_collect(h, mark, bytes);
+  h->pot_bytes -= former;
 }
 
 // the resident coordinates, from and to the caller's memory
@@ -1663,7 +1687,13 @@ int minim_gpu_instance_set_fixed(minim_gpu_handle h, const int* idof, size_t n) 
       f[idof[i]] = 1;
     }
     h->fixed = n ? f : std::vector<unsigned char>();
+    void* former = const_cast<unsigned char*>(h->d.fixed);
     h->d.fixed = h->own_upload(h->fixed);
+    if (former) {
+      h->owned.erase(std::find(h->owned.begin(), h->owned.end(), former));
+      dfree(former);
+      h->pot_bytes -= h->n;
+    }
     if (h->kind == MINIM_GPU_BAH) upload_bah_arrays(h);
     CK(cudaStreamSynchronize(dev().s));
   });

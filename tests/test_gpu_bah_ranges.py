@@ -1,6 +1,7 @@
 """BarAndHinge at the ends of its ranges: FP32 forces of very unequal elements
 at one vertex, hinge angles on both sides of their rule, a vertex of thousands
-of elements, the memory a request holds.
+of elements, the memory instances and
+requests hold.
 """
 import time
 
@@ -94,6 +95,19 @@ def test_hub(n):
     e, g = inst.energy_gradient(y)
     tol = 1e-12 * max(1.0, n / 40)
     assert abs(e - eo) <= tol * abs(eo) and np.max(np.abs(g - go)) <= tol * np.max(np.abs(go))
+
+
+def test_set_fixed_gives_memory_back():
+    """Fixing other coordinates builds the element lists anew; the old ones go."""
+    flat, tris, _ = sheet(200, seed=3)
+    inst = runtime.Instance(abi.bar_and_hinge(triangulation=tris, rigidity=(1, 0.01)), flat)
+    inst.set_fixed([0, 1, 2])
+    inst.energy()
+    free = torch.cuda.mem_get_info()[0]
+    for k in range(60):
+        inst.set_fixed(list(range(3 * k, 3 * k + 9)))
+    # a sheet of 40,000 vertices holds some 30 MB
+    assert free - torch.cuda.mem_get_info()[0] < 256 << 20
 
 
 @pytest.mark.parametrize("explicit", [False, True])
