@@ -765,7 +765,7 @@ int grid_error(minim_gpu_instance_s* h) {
 
 int rule_threads(int kk, const InstDesc& d);
 int lj_batch_rows(const MinParams& mp);
-bool single_shape(int kk, const InstDesc& d, int* threads, int* csize);
+bool single_shape(int kk, const InstDesc& d, int prec, int* threads, int* csize);
 void launch_single(int kk, int threads, int csize, const InstDesc* d_inst, int* counter, const InstDesc& d,
                    cudaStream_t s);
 
@@ -777,7 +777,7 @@ void launch_single(int kk, int threads, int csize, const InstDesc* d_inst, int* 
 bool eval_small(minim_gpu_instance_s* h, const double* x, double* e, double* g) {
   Dev& D = need_dev();
   int threads = 0, csize = 0;
-  if (!h->hx || h->kk == K_PF || !single_shape(h->kk, h->d, &threads, &csize)) return false;
+  if (!h->hx || h->kk == K_PF || !single_shape(h->kk, h->d, MINIM_PREC_FP64, &threads, &csize)) return false;
   const size_t n = h->n;
   if (!h->h_xg) h->h_xg = (double*)pinned().alloc(2 * n * sizeof(double));
   if (!h->h_xg) return false;
@@ -974,7 +974,8 @@ void do_minimise(minim_gpu_instance_s* h, const minim_gpu_minimiser_params& mp, 
   // pass's controller, which has no step cap (Lbfgs::setMaxStep)
   const bool dual = stepped_ok && dual_cfg() && mp.max_step == 0;
   int s_threads = 0, s_csize = 0;
-  const bool small = !stepped_ok && single_shape(h->kk, h->d, &s_threads, &s_csize);
+  const int prec = mp.method == MINIM_ANNEAL ? MINIM_PREC_FP64 : mp.precision;
+  const bool small = !stepped_ok && single_shape(h->kk, h->d, prec, &s_threads, &s_csize);
   WsLayout L = ws_layout(h->n, mp, dual);
   // the state record, then (in one upload with it) the descriptor and the
   // instance counter of a batch launch
@@ -1288,34 +1289,49 @@ void launch_shape(int kk, const Shape& sh, const InstDesc* d_insts, int ninst, i
   g_launches++;
 }
 
-// The launch shape of a single minimisation small enough for one CTA or one
-// cluster: their barriers and reductions (well under a microsecond, two to
-// three in a cluster) replace the whole GPU's (about six), until the SMs
-// that the grid adds are worth more.  Microseconds an L-BFGS iteration on the
-// grid and with the shape chosen here (FP32 stage; FP64 in brackets):
-// Lennard-Jones N = 13 108, 29 (99, 49); 256 173, 44 (298, 55); 1500, on the
-// grid, 86 against 103 (158, 477); binary PhaseField 64^2 119, 62 (105, 64),
-// 128^2 120, 77 (102, 118), 256^2 119 against 140; channel 61 x 47 154, 97
-// (108, 74), 128^2 156 against 152 (115, 148); three fluids 64^2 146, 90
-// (201, 142), 128^2 148 against 147 (202, 341).
-bool single_shape(int kk, const InstDesc& d, int* threads, int* csize) {
+// The launch shape of a single minimisation or evaluation small enough for one
+// CTA or one cluster: their barriers and reductions (well under a microsecond,
+// two to three in a cluster) replace the whole GPU's (about six), until the SMs
+// that the grid adds are worth more -- in FP64, where the arithmetic sets the
+// time, much earlier than in FP32.  `prec` is the run's precision; evaluations
+// and annealing are FP64.  Microseconds an L-BFGS iteration on the grid and with
+// the shape chosen here, FP32; FP64; mixed near the minimum (half or more of the
+// iterations in the FP64 stage):
+//   Lennard-Jones N = 13 104, 25; 103, 30; 141, 35.  256 88, 30; 99, 49.  512 86,
+//   34; 115, 99.  640 85, 50; 121, 151; 170, 156.  896 86, 71; 129, 250; 197, 286.
+//   1024 86, 61; 132, 276.  With a cutoff (15 iterations): 512 cluster 810; 1650.
+//   768 1330; 2970.  1024 1790; 4450, the grid at 1200 1350; 1900.
+//   Binary PhaseField 64^2 87, 38; 108, 68.  96^2 90, 44; 108, 105; 108, 85.  112^2
+//   94, 48; 106, 119; 106, 89.  128^2 87, 47; 107, 130; 109, 101.  141^2 93, 62; 106,
+//   147; 109, 114.
+//   Channels 90^2 112, 63; 122, 100; 113, 75.  100^2 109, 67; 119, 139; 115, 96.
+//   Three fluids 64^2 132, 66; 175, 109; 177, 112.  89^2 128, 78; 164, 139; 183, 119.
+//   Sheets of 300 dofs (one CTA) 80, 28; 123, 71; 243, 81.  972 (one CTA) 84, 45; 129,
+//   186; 230, 155.  1083 (cluster) 84, 46; 128, 128; 225, 132.  3888 84, 47; 168, 129.
+// Evaluations with the gradient, the call: N = 256 50, 31; 512 60, 56; 640 60, 82;
+// 1024 63, 156; sheets of 588 dofs 62, 55 (one CTA); 972 63, 82 (one CTA); 1083 63, 58.
+bool single_shape(int kk, const InstDesc& d, int prec, int* threads, int* csize) {
+  const bool fp32 = prec == MINIM_PREC_FP32, fp64 = prec == MINIM_PREC_FP64;
   if (kk == K_LJ) {
     const int n = d.lj.np;
     *threads = n <= 96 ? 128 : 256;
     *csize = n <= 96 ? 1 : 8;
-    return n <= 1024;
+    if (d.lj.rc2 > 0) return n <= (fp32 ? 768 : 512);
+    return n <= (fp32 ? 1024 : (fp64 ? 512 : 640));
   }
   const int n = d.ndof;
   *threads = 512;
   *csize = 8;
   if (kk == K_PF1 || kk == K_BAH) {
-    if (n <= 1024) {
+    if (n <= (kk == K_BAH && fp64 ? 600 : 1024)) {
       *threads = 256;
       *csize = 1;
     }
-    return n <= (kk == K_BAH ? 4096 : 20000);
+    if (kk == K_BAH) return n <= 4096;
+    return n <= (fp32 ? 20000 : (fp64 ? 9216 : 16384));
   }
-  return n <= (d.pf.nfluid > 1 ? 24000 : 12000);
+  if (d.pf.nfluid > 1) return n <= 24000;
+  return n <= (fp64 ? 8192 : 12000);
 }
 void launch_single(int kk, int threads, int csize, const InstDesc* d_inst, int* counter, const InstDesc& d,
                    cudaStream_t s) {
