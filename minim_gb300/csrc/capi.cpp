@@ -766,6 +766,8 @@ int grid_error(minim_gpu_instance_s* h) {
 int rule_threads(int kk, const InstDesc& d);
 int lj_batch_rows(const MinParams& mp);
 bool single_shape(int kk, const InstDesc& d, int prec, int* threads, int* csize);
+bool single_fits(int kk, const InstDesc& d, int threads, int csize);
+bool clusters_cfg();
 void launch_single(int kk, int threads, int csize, const InstDesc* d_inst, int* counter, const InstDesc& d,
                    cudaStream_t s);
 
@@ -778,6 +780,7 @@ bool eval_small(minim_gpu_instance_s* h, const double* x, double* e, double* g) 
   Dev& D = need_dev();
   int threads = 0, csize = 0;
   if (!h->hx || h->kk == K_PF || !single_shape(h->kk, h->d, MINIM_PREC_FP64, &threads, &csize)) return false;
+  if (csize > 1 && !clusters_cfg()) return false;
   const size_t n = h->n;
   if (!h->h_xg) h->h_xg = (double*)pinned().alloc(2 * n * sizeof(double));
   if (!h->h_xg) return false;
@@ -794,7 +797,10 @@ bool eval_small(minim_gpu_instance_s* h, const double* x, double* e, double* g) 
   }
   io.g = g ? h->h_xg + n : nullptr;
   io.e = &h->h_out->e;
-  CK((cudaError_t)kern(h->kk).api_eval(&h->d, &io, threads, csize, group_smem(h->kk, &h->d, 1, threads), D.s));
+  if (kern(h->kk).api_eval(&h->d, &io, threads, csize, group_smem(h->kk, &h->d, 1, threads), D.s) != cudaSuccess) {
+    cudaGetLastError();  // the device cannot hold the cluster: the grid
+    return false;
+  }
   g_launches++;
   CK(cudaStreamSynchronize(D.s));
   if (g) std::memcpy(g, h->h_xg + n, n * sizeof(double));
@@ -975,7 +981,8 @@ void do_minimise(minim_gpu_instance_s* h, const minim_gpu_minimiser_params& mp, 
   const bool dual = stepped_ok && dual_cfg() && mp.max_step == 0;
   int s_threads = 0, s_csize = 0;
   const int prec = mp.method == MINIM_ANNEAL ? MINIM_PREC_FP64 : mp.precision;
-  const bool small = !stepped_ok && single_shape(h->kk, h->d, prec, &s_threads, &s_csize);
+  const bool small = !stepped_ok && single_shape(h->kk, h->d, prec, &s_threads, &s_csize) &&
+                     single_fits(h->kk, h->d, s_threads, s_csize);
   WsLayout L = ws_layout(h->n, mp, dual);
   // the state record, then (in one upload with it) the descriptor and the
   // instance counter of a batch launch
@@ -1332,6 +1339,15 @@ bool single_shape(int kk, const InstDesc& d, int prec, int* threads, int* csize)
   }
   if (d.pf.nfluid > 1) return n <= 24000;
   return n <= (fp64 ? 8192 : 12000);
+}
+// Whether the device can hold such a cluster (MINIM_GPU_CLUSTERS=0: as if it
+// could not); without, single minimisations run on the grid.
+bool clusters_cfg() {
+  const char* e = std::getenv("MINIM_GPU_CLUSTERS");
+  return !(e && e[0] == '0');
+}
+bool single_fits(int kk, const InstDesc& d, int threads, int csize) {
+  return csize == 1 || (clusters_cfg() && shape_slots(kk, Shape{threads, csize}, group_smem(kk, &d, 1, threads)) > 0);
 }
 void launch_single(int kk, int threads, int csize, const InstDesc* d_inst, int* counter, const InstDesc& d,
                    cudaStream_t s) {

@@ -91,3 +91,20 @@ def test_evaluation_sides(case):
         e, g = inst.energy_gradient(*args)
         assert abs(e - eo) <= 1e-11 * abs(eo) and np.max(np.abs(g - go)) <= 1e-10 * np.max(np.abs(go))
         assert abs(inst.energy(*args) - eo) <= 1e-11 * abs(eo)
+
+
+@pytest.mark.parametrize("case", [_lj(300), _lj(300, 2.5), _pf1(40, 40), _wall(30, 31), _sheet(30)], ids=range(5))
+def test_without_clusters(case, monkeypatch):
+    """A device that cannot hold a cluster of eight runs small instances on the grid."""
+    p, x0, x = case
+    x = x0 if x is None else x
+    inst, o = runtime.Instance(p, x0), Oracle(p, x0)
+    monkeypatch.setenv("MINIM_GPU_CLUSTERS", "0")
+    eo, go = o.energy_gradient(x)
+    e, g = inst.energy_gradient(x)
+    assert abs(e - eo) <= 1e-11 * abs(eo) and np.max(np.abs(g - go)) <= 1e-10 * np.max(np.abs(go))
+    inst.coords = x
+    before = runtime.launch_count()
+    r = inst.minimise(abi.minimiser("lbfgs", tol=0.0, max_iter=100, precision="fp64"))
+    assert r.iter >= 100 and runtime.launch_count() - before > 1
+    assert abs(o.energy(inst.coords) - r.energy) <= 1e-9 * max(abs(r.energy), 1e-3)
