@@ -331,7 +331,8 @@ int minim_gpu_pf_setup(int kind, const minim_gpu_pf_params* q, const double* x0,
  * evaluation of the same point (the reference's State::energyGradient,
  * src/State.cpp:134-192, is FP64 throughout).  path:
  *   MINIM_EVAL_FP32_GRID   FP32 coordinates, the single-instance kernels (whole GPU)
- *   MINIM_EVAL_FP32_CTA    FP32 coordinates, the batch kernels (one CTA per instance)
+ *   MINIM_EVAL_FP32_CTA    FP32 coordinates, the batch kernels (one CTA per instance;
+ *                          of L-BFGS where methods differ: Lennard-Jones pairs)
  *   MINIM_EVAL_FP64S_GRID  FP64 coordinates with the FP64 stage's arithmetic
  *                          (double-float where the minimiser uses it), whole GPU
  *   MINIM_EVAL_FP64S_CTA   the same on one CTA

@@ -932,6 +932,7 @@ void do_eval_kernel(minim_gpu_instance_s* h, int path, const double* x, const do
     d.X32[1] = vec(4);
     d.mp = MinParams{};
     d.mp.method = MINIM_LBFGS;
+    d.lj.rows = lj_batch_rows(d.mp);  // one CTA: a batched L-BFGS run's evaluators
     EvalIO io{};
     io.x = h->d_tmp;
     io.e = h->d_e;
@@ -946,8 +947,8 @@ void do_eval_kernel(minim_gpu_instance_s* h, int path, const double* x, const do
     if (path == MINIM_EVAL_FP32_GRID || path == MINIM_EVAL_FP64S_GRID) {
       launch_grid(h, OP_EVAL_STAGE, 0);
     } else {
-      const int thr = rule_threads(h->kk, h->d);
-      CK((cudaError_t)kern(h->kk).cta_eval(h->d_desc, h->d_io, thr, group_smem(h->kk, &h->d, 1, thr), D.s));
+      const int thr = rule_threads(h->kk, d);
+      CK((cudaError_t)kern(h->kk).cta_eval(h->d_desc, h->d_io, thr, group_smem(h->kk, &d, 1, thr), D.s));
       g_launches++;
     }
     CK(cudaMemcpyAsync(&ev[0], h->d_e, sizeof(double), cudaMemcpyDeviceToHost, D.s));

@@ -116,3 +116,19 @@ def test_fp32_energy_keeps_small_terms():
         inst = runtime.Instance(abi.lj(), some.ravel(), fixed=list(range(some.size)))
         r = inst.minimise(abi.minimiser("lbfgs", tol=1e-9, max_iter=5, precision="fp32"))
         assert abs(r.energy - exact * sites / 150) <= sites * 4 * 15 * 1e-6, (sites, r.energy)
+
+
+@pytest.mark.parametrize("n", [13, 40, 64, 90, 200, 256, 400])
+def test_cta_evaluation_is_the_batch_kernels(n):
+    """The stage evaluations on one CTA run the pair code of a batched L-BFGS
+    run: the energies of a run that cannot move (every coordinate fixed) agree
+    but for the order of a few FP64 additions."""
+    x = _grid(n, seed=n).ravel().astype(np.float32).astype(np.float64)
+    for precision, path in (("fp32", abi.EVAL_FP32_CTA), ("mixed", abi.EVAL_FP64S_CTA)):
+        inst = runtime.Instance(abi.lj(), x, fixed=list(range(3 * n)))
+        b = runtime.Batch()
+        b.add(inst, abi.minimiser("lbfgs", tol=1e-9, max_iter=5, precision=precision))
+        r = b.run(64 if n <= 96 else (128 if n <= 192 else 256))[0]
+        assert precision == "fp32" or r.fp64_iters > 0
+        e, _ = inst.eval_kernel(path, x)
+        assert abs(e - r.energy) <= 4e-15 * abs(e), (precision, e, r.energy)
