@@ -1,5 +1,6 @@
 """Lennard-Jones evaluators at the ends of their ranges: coordinates in large
-units, sums of many comparable terms, energies of very unequal pairs.
+units, sums of many comparable terms, energies of very unequal pairs, cutoffs
+seen from far out, coordinates that are not finite.
 """
 import numpy as np
 import pytest
@@ -132,3 +133,50 @@ def test_cta_evaluation_is_the_batch_kernels(n):
         assert precision == "fp32" or r.fp64_iters > 0
         e, _ = inst.eval_kernel(path, x)
         assert abs(e - r.energy) <= 4e-15 * abs(e), (precision, e, r.energy)
+
+
+def test_cutoff_from_far_out():
+    """Pairs a millionth inside and outside the cutoff, 1e8 from the origin: the
+    pairs counted are those of the FP64 criterion.  (Coordinates are good to
+    2^-48 of 1e8 there, 4e-7: an energy of -0.0163 a pair to 4e-8.)"""
+    for n in (32, 300, 2100):
+        m = n // 2
+        pts = np.zeros((2 * m, 3))
+        pts[0::2, 0] = pts[1::2, 0] = 1e8 + 16.0 * np.arange(m)
+        pts[1::2, 0] += 2.5 + np.where(np.arange(m) % 2 == 0, -1e-6, 1e-6)
+        p = abi.lj(cutoff=2.5)
+        inst, o = runtime.Instance(p, pts.ravel()), Oracle(p, pts.ravel())
+        eo = o.energy()
+        assert abs(eo + 0.0163169 * ((m + 1) // 2)) < 1e-5 * m
+        e, _ = inst.energy_gradient(pts.ravel())
+        assert abs(e - eo) <= 4e-7 * m
+        assert abs(inst.energy(pts.ravel()) - eo) <= 4e-7 * m
+
+
+@pytest.mark.parametrize("n", [13, 40, 80, 300, 2100])
+@pytest.mark.parametrize("cutoff", [0.0, 2.5])
+def test_not_finite(n, cutoff):
+    """A NaN coordinate makes the energy NaN, and its particle's force; without a
+    cutoff everyone's.  A particle at infinity is outside every cutoff."""
+    p = abi.lj(cutoff=cutoff)
+    x = _grid(n)
+    bad = x.copy()
+    bad[n // 2, 1] = np.nan
+    inst = runtime.Instance(p, x.ravel())
+    e, g = inst.energy_gradient(bad.ravel())
+    assert np.isnan(e) and np.isnan(inst.energy(bad.ravel()))
+    g = g.reshape(n, 3)
+    assert np.isnan(g[n // 2, 1])
+    if cutoff == 0:
+        assert np.all(np.isnan(g[:, 1]))
+        return
+    away = np.sum((np.delete(x, n // 2, 0) - x[n // 2]) ** 2, axis=1) > 9
+    assert np.all(np.isfinite(np.delete(g, n // 2, 0)[away]))
+    far = x.copy()
+    far[n // 2, 1] = np.inf
+    rest = np.delete(x, n // 2, 0)
+    eo, go = Oracle(p, rest.ravel()).energy_gradient()
+    e, g = inst.energy_gradient(far.ravel())
+    assert abs(e - eo) <= 1e-12 * abs(eo) and abs(inst.energy(far.ravel()) - eo) <= 1e-12 * abs(eo)
+    others = np.delete(g.reshape(n, 3), n // 2, 0)
+    assert np.max(np.abs(others.ravel() - go)) <= 1e-12 * n * np.max(np.abs(go))

@@ -108,3 +108,39 @@ def test_without_clusters(case, monkeypatch):
     r = inst.minimise(abi.minimiser("lbfgs", tol=0.0, max_iter=100, precision="fp64"))
     assert r.iter >= 100 and runtime.launch_count() - before > 1
     assert abs(o.energy(inst.coords) - r.energy) <= 1e-9 * max(abs(r.energy), 1e-3)
+
+
+def test_page_locked_coordinates():
+    """Coordinates of many small instances share chunks of page-locked memory that
+    are used again and given back: everyone's own stay as they were, also past
+    the pool's 256 MB, where they live on the device."""
+    p = abi.lj(ndim=2)
+    rng = np.random.default_rng(5)
+    base = np.stack(np.meshgrid(np.arange(64), np.arange(32), indexing="ij"), -1).reshape(-1, 2) * 1.1
+    held = {}
+
+    def make(k, n):
+        x = (base[:n] + rng.uniform(-0.05, 0.05, (n, 2))).ravel()
+        held[k] = (runtime.Instance(p, x), x)
+
+    for k in range(300):
+        make(k, int(rng.integers(1, 2049)))
+    for k in list(held)[::2]:
+        held.pop(k)[0].close()
+    for k in range(300, 600):
+        make(k, int(rng.integers(1, 2049)))
+    for inst, x in held.values():
+        assert np.array_equal(inst.coords, x)
+    for k in list(held)[:-1]:
+        held.pop(k)[0].close()
+    (inst, x), = held.values()
+    e0, g0 = inst.energy_gradient()
+    many = [runtime.Instance(p, base.ravel() + 1e-3 * k) for k in range(8300)]
+    for k, h in enumerate(many):
+        assert np.array_equal(h.coords, base.ravel() + 1e-3 * k)
+    r = [h.minimise(abi.minimiser("lbfgs", tol=0.0, max_iter=3, precision="fp64")) for h in (many[0], many[-1])]
+    assert abs(r[0].energy - r[1].energy) <= 1e-9 * abs(r[0].energy)
+    e, g = inst.energy_gradient()
+    assert e == e0 and np.array_equal(g, g0)
+    for h in many:
+        h.close()
