@@ -99,12 +99,23 @@ struct StoreEmit64 {
   }
 };
 
+// Lennard-Jones with a cutoff: largest cluster whose rows test every pair instead
+// of building a cell list, by team.  The rows' N^2 tests are what the team's
+// threads divide; the list costs passes, barriers and, per particle, what its
+// neighbourhood holds, so the line lies where a dilute gas (density 0.02) is
+// even -- a crystal gains from rows further up.  15 L-BFGS iterations, rows /
+// cell list, FP32: one CTA N = 256 gas 1.00 / 1.63 ms, crystal 1.13 / 6.46; 512 2.5
+// / 2.9, 3.3 / 11.8; 768 4.9 / 3.8, 6.8 / 19; 2048 28 / 11, 39 / 48.  A cluster of
+// eight 512 0.75 / 1.9, 0.81 / 6.6; 1024 1.40 / 1.96, 1.8 / 6.6; 1500 2.7 / 2.5, 3.1 /
+// 7.3; 2048 3.9 / 2.4, 5.6 / 8.3.  The grid 2048 1.5 / 3.6, 1.5 / 11.
+template <class Team>
+__host__ __device__ constexpr int lj_cut_rows() {
+  return !Team::kGrid ? 512 : (Team::kCluster ? 1024 : 2048);
+}
+
 // Work counters and phase timers are only read from thread 0 (which stores
 // the state): only thread 0 updates them, so the other threads issue no FP64
 // instruction for them (FP64 runs at 1/64 of the FP32 rate on GB300).
-// Lennard-Jones with a cutoff: largest cluster evaluated without a cell list
-constexpr int kLjCutRows = 2048;
-
 #define MG_ACCT(ctr, expr)            \
   do {                                \
     if (threadIdx.x == 0) (ctr) += (expr); \
@@ -182,10 +193,8 @@ struct Runner {
   __device__ EPart<T> pot_eval(CView<T> cv, T* xw, Emit& em, bool want_e, bool want_g) {
     if constexpr (KIND == K_LJ) {
       if (in.lj.rc2 > 0) {
-        // with a cutoff: rows that skip the pairs outside it, up to
-        // kLjCutRows particles (the cell list's passes and barriers cost more
-        // there), the cell list above
-        if (in.lj.np <= kLjCutRows) {
+        // with a cutoff: rows that skip the pairs outside it, or the cell list
+        if (in.lj.np <= lj_cut_rows<Team>()) {
           if (want_g) return lj_rows<T, true>(tm, in.lj, cv, xw, &em, smem_pot);
           if (!xw) return lj_energy<T, true>(tm, in.lj, cv, smem_pot);
         }

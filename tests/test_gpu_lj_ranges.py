@@ -180,3 +180,25 @@ def test_not_finite(n, cutoff):
     assert abs(e - eo) <= 1e-12 * abs(eo) and abs(inst.energy(far.ravel()) - eo) <= 1e-12 * abs(eo)
     others = np.delete(g.reshape(n, 3), n // 2, 0)
     assert np.max(np.abs(others.ravel() - go)) <= 1e-12 * n * np.max(np.abs(go))
+
+
+@pytest.mark.parametrize("spacing", [1.08, 2.4])
+@pytest.mark.parametrize("n,ctas", [(511, 1), (512, 1), (513, 1), (700, 1), (1023, 8), (1024, 8), (1025, 8), (1100, 2),
+                                    (2047, 0), (2048, 0), (2049, 0)])
+def test_cutoff_rows_and_cells(n, ctas, spacing):
+    """On either side of where rows end and the cell list begins, one CTA, cluster
+    and grid: the energy of a run that cannot move is the oracle's, dense and
+    dilute."""
+    p = abi.lj(cutoff=2.5)
+    x = (_grid(n) * (spacing / 1.08)).ravel().astype(np.float32).astype(np.float64)
+    eo = Oracle(p, x).energy()
+    inst = runtime.Instance(p, x, fixed=list(range(3 * n)))
+    for precision, tol in (("fp32", 2e-6), ("fp64", 1e-12)):
+        mp = abi.minimiser("lbfgs", tol=1e-9, max_iter=5, precision=precision)
+        if ctas:
+            b = runtime.Batch()
+            b.add(inst, mp)
+            r = b.run(256, ctas)[0]
+        else:
+            r = inst.minimise(mp)
+        assert abs(r.energy - eo) <= tol * abs(eo)
