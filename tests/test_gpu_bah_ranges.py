@@ -1,7 +1,7 @@
 """BarAndHinge at the ends of its ranges: FP32 forces of very unequal elements
 at one vertex, hinge angles on both sides of their rule, a vertex of thousands
 of elements, the memory instances and
-requests hold.
+requests hold, a free vertex that is nowhere.
 """
 import time
 
@@ -130,3 +130,20 @@ def test_server_budget_counts_the_elements(explicit):
         (_, r), = srv.poll()
         assert (r.status == abi.RES_REJECTED) == (status == abi.RES_REJECTED)
         srv.close()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_free_vertex_at_no_height(bad):
+    """A vertex in no triangle still carries the external force's element: without
+    a force its energy is 0 z, no number where z is none."""
+    flat, tris, pert = sheet(6, seed=2)
+    x0 = np.concatenate([flat, [9.0, 9.0, 0.5]])
+    x = np.concatenate([pert, [9.0, 9.0, 0.5]])
+    inst = runtime.Instance(abi.bar_and_hinge(triangulation=tris, rigidity=(1, 0.01)), x0)
+    assert np.isfinite(inst.energy(x))
+    x[-1] = bad
+    assert np.isnan(inst.energy(x))
+    e, g = inst.energy_gradient(x)
+    assert np.isnan(e) and np.all(np.isfinite(g))
+    for path in (abi.EVAL_FP32_GRID, abi.EVAL_FP32_CTA, abi.EVAL_FP64S_GRID, abi.EVAL_FP64S_CTA):
+        assert np.isnan(inst.eval_kernel(path, x)[0]), path
