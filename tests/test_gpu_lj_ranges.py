@@ -202,3 +202,18 @@ def test_cutoff_rows_and_cells(n, ctas, spacing):
         else:
             r = inst.minimise(mp)
         assert abs(r.energy - eo) <= tol * abs(eo)
+
+
+@pytest.mark.parametrize("ndim", [2, 3])
+@pytest.mark.parametrize("x", [0.3, np.nan, np.inf, -np.inf, 1e200, 1e30])
+def test_single_particle(x, ndim):
+    """One particle has no pair: no energy and no force wherever it is."""
+    pos = np.array([0.5, x, -0.2])[:ndim]
+    inst = runtime.Instance(abi.lj(ndim=ndim), pos)
+    e, g = inst.energy_gradient(pos)
+    assert e == 0 and np.all(g == 0) and inst.energy(pos) == 0
+    for precision in ("fp32", "mixed", "fp64"):
+        for method in (dict(method="lbfgs"), dict(method="fire", dt_max=0.02)):
+            inst.coords = pos
+            r = inst.minimise(abi.minimiser(max_iter=5, tol=1e-6, precision=precision, **method))
+            assert r.status == abi.RES_CONVERGED and r.energy == 0
