@@ -217,3 +217,26 @@ def test_single_particle(x, ndim):
             inst.coords = pos
             r = inst.minimise(abi.minimiser(max_iter=5, tol=1e-6, precision=precision, **method))
             assert r.status == abi.RES_CONVERGED and r.energy == 0
+
+
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("unit", [1e6, 1e15])
+def test_particle_far_along_an_axis(unit, axis):
+    """A particle far out along one coordinate meets nothing, no padding either
+    (which stood at (1e6 k, 0, 0)): the others' energy and forces are theirs alone."""
+    n = 80
+    p = abi.lj()
+    x = _grid(n, seed=6)
+    x[n - 1] = 0.0
+    eo, go = Oracle(p, x[:n - 1].ravel()).energy_gradient()
+    inst = runtime.Instance(p, x.ravel())
+    for k in range(n, 98):
+        x[n - 1, axis] = k * unit
+        tol = 1e-12 + (n * (5.0 / unit) ** 6 if unit < 1e10 else 0.0)
+        e, g = inst.energy_gradient(x.ravel())
+        assert abs(e - eo) <= tol * abs(eo) and np.max(np.abs(g[:-3] - go)) <= 1e-12 * n * np.max(np.abs(go))
+        for path, ge, ee in ((abi.EVAL_FP32_CTA, 1e-5, 2e-6), (abi.EVAL_FP64S_CTA, 2e-7, 1e-12)):
+            xs = x.astype(np.float32).astype(np.float64) if path == abi.EVAL_FP32_CTA else x
+            es, gs = Oracle(p, xs[:n - 1].ravel()).energy_gradient()
+            e, g = inst.eval_kernel(path, xs.ravel())
+            assert abs(e - es) <= ee * abs(es) and np.max(np.abs(g[:-3] - gs)) <= ge * np.max(np.abs(gs)), (k, path)
