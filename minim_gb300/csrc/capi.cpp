@@ -772,10 +772,10 @@ void launch_single(int kk, int threads, int csize, const InstDesc* d_inst, int* 
                    cudaStream_t s);
 
 // The evaluation of a small instance by one CTA or cluster: one launch that
-// reads page-locked host memory (Lennard-Jones: each coordinate once; the
-// others' stencils and gathers from a device copy) and writes E and g there.
-// A cluster of 13: 68 us with six copies and memsets around a launch of the
-// whole GPU.  Now 22 us.
+// reads page-locked host memory (Lennard-Jones: every CTA stages each coordinate
+// once, eight reads of at most 12 KB on a cluster; the others' stencils and
+// gathers from a device copy) and writes E and g there.  A cluster of 13: 68 us
+// with six copies and memsets around a launch of the whole GPU, 21 us so.
 bool eval_small(minim_gpu_instance_s* h, const double* x, double* e, double* g) {
   Dev& D = need_dev();
   int threads = 0, csize = 0;
@@ -1487,10 +1487,12 @@ std::vector<Shape> batch_shapes(const std::vector<InstDesc>& descs, const std::v
 }
 
 // The one-CTA Lennard-Jones evaluators of a batched instance (PotLJ::rows):
-// L-BFGS and gradient descent keep the tile pairs by rounds -- 384 clusters of
-// 13 to 400 particles by L-BFGS took 33 ms of kernel time with them and 32
-// with the others, their line searches spending the time; FIRE 32 and 30 ms,
-// annealing (1024 clusters of 38) 75 and 38 ms.
+// L-BFGS and gradient descent keep the tile pairs by rounds.  Kernel time of
+// L-BFGS batches by rounds and with the others: 384 crystals of 13 to 400
+// particles 33.7 ms and 29.1, 256 random clusters 201 and 232; 304 crystals of 33 to
+// 64 8.6 and 7.2, 65 to 96 9.2 and 13.1, 193 to 256 19.9 and 25.4, 321 to 400 40.0 and
+// 36.4 -- neither serves all.  FIRE 32 and 27 ms, annealing (1024 clusters of 38) 75
+// and 32 ms.
 int lj_batch_rows(const MinParams& mp) { return mp.method == MINIM_FIRE || mp.method == MINIM_ANNEAL; }
 
 // Runs the given instances with the batch kernels: one launch per (kernel

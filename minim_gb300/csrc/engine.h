@@ -63,8 +63,9 @@ constexpr size_t kLjSmemBudget = 48 * 1024, kLjSmemRows = 98 * 1024;
 // 36.1 / 33.3, 300 195 / 148.
 constexpr int kLjRowsMax = 64;
 // FP32 tile pairs go two i tiles a unit (lj_eval_dealt2) above this size, where
-// there are enough units for eight warps: a FIRE iteration of N = 200 21.7 us by
-// single tiles against 21.9, 300 32.9 / 32.3, 400 47.2 / 44.5.
+// there are enough units for eight warps: a FIRE iteration, 304 clusters of 256
+// threads, N = 65 12.5 us by single tiles against 13.4, 200 20.0 / 20.8, 257 27.7 /
+// 26.6, 300 31.2 / 30.7, 384 40.3 / 37.8, 400 46.0 / 43.0.
 constexpr int kLjDealt2Min = 256;
 MG_HD inline bool lj_dealt_fits(int np, int nwarps, bool fp64, int rows) {
   if (!rows) return !fp64 && lj_dealt_bytes(np, nwarps, fp64) <= kLjSmemBudget;
@@ -225,12 +226,12 @@ struct MinScalars {
   // device time (ns, block 0) in gradient evaluations, line-search trial
   // evaluations and L-BFGS direction passes
   double tphase[3];
-  // batch kernels: %globaltimer when a CTA first took the instance and when
-  // one last stored it (ns)
   // FIRE without a line search: the next iteration's velocity update, decided
   // with the last gradient (fire_decide)
   int fire_ready, fire_mix;
   float fire_f1, fire_f2, fire_dt;
+  // batch kernels: %globaltimer when a CTA first took the instance and when
+  // one last stored it (ns)
   unsigned long long t_first, t_last;
 };
 
